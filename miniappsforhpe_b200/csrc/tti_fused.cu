@@ -2197,15 +2197,20 @@ unsigned cta_count(const Layout& L, Split sp)
     return (unsigned)(T + (T * (L.nz() - sp.ztop) + sp.bz - 1) / sp.bz);
 }
 
-// Planes per CTA worth trying: whole-column chunks ceil(nz/n), and shares
-// that give every SM one, two, ... equal parts of the work; at least 8.
+// Planes per CTA worth trying: whole-column chunks ceil(nz/n) of at least 2
+// planes, and shares of at least 8 that give every SM one, two, ... equal
+// parts of the work.  A 2-plane chunk computes 2 planes out of 16, yet on a
+// grid of few columns the SMs would otherwise idle: 48x40x40 (6 columns), 2
+// planes against 8: forward 21 against 38 us, adjoint 41 against 59 us,
+// imaging 47 against 64 us; a chunk of 1 plane (two waves) is slower again
+// (74 us adjoint).
 std::vector<int> plane_candidates(const Layout& L)
 {
     std::vector<int> c;
     const int nz = L.nz();
     for (int nch = 1; nch <= nz; ++nch) {
         const int bz = (nz + nch - 1) / nch;
-        if (bz < 8 && nch > 1) break;
+        if (bz < 2 && nch > 1) break;
         c.push_back(bz);
         if (nz % nch == 0) c.push_back(nz / nch);
     }
