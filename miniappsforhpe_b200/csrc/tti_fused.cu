@@ -657,6 +657,12 @@ __global__ void __launch_bounds__(NT, 1)
 // 128-bit shared loads.  The transposed-model temporaries of a plane are
 // formed once per staging position that needs them, in passes whose role
 // (which temporaries a position feeds) is uniform per warp.
+//
+// SKIP: the pipeline fill's planes (seven either side of the outputs) form
+// only what outputs take from them: zz at the column, and yz, zx from the
+// four nearest.  On small grids, whose chunks are short, most planes are such;
+// on long chunks the branches cost more than they save, because the compiler
+// no longer overlaps the phases (see adj_skips_fill).
 struct AdjParams {
     float* pout;
     float* qout;
@@ -712,11 +718,11 @@ static_assert(adj_smem(true) <= 227 * 1024, "adjoint staging and tiles fit one C
 
 struct AdjMaps {
     CUtensorMap p, q;  // box PW x PH
-    CUtensorMap ma;    // 4D (4, x, y, z), box 4 x PW x PH
-    CUtensorMap mb;    // TTI: 4D like ma; VTI: irho, box PW x PH
+    CUtensorMap ma;    // float4 cells, box PW x PH (by rows in the skipping form)
+    CUtensorMap mb;    // TTI: like ma; VTI: irho, box PW x PH
 };
 
-template <bool TTI>
+template <bool TTI, bool SKIP>
 __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__ AdjMaps tm, const AdjParams a)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -756,7 +762,7 @@ __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__
     int gbase = 0;  // planes consumed by earlier segments
     WorkRange wr(L, a.bz, a.ztop);
     for (Segment sg; wr.next(sg); gbase += sg.len + 2 * LAG) {
-    const int x0 = sg.x0, y0 = sg.y0, zs = sg.zs;
+    const int x0 = sg.x0, y0 = sg.y0, zs = sg.zs, ze = sg.zs + sg.len - 1;
     const int ntot = sg.len + 2 * LAG;
     const int x = x0 + tx, y = y0 + ty;
     const bool owner = (x <= L.ixend) && (y <= L.iyend);
@@ -772,9 +778,15 @@ __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__
         mbar_expect_tx(&bars[sl], (uint32_t)STAGE);
         tma_load_3d(dst, &tm.p, x0 - 8, y0 - 8, z, &bars[sl]);
         tma_load_3d(dst + ADJ_F1, &tm.q, x0 - 8, y0 - 8, z, &bars[sl]);
-        tma_load_4d(dst + 2 * ADJ_F1, &tm.ma, 0, x0 - 8, y0 - 8, z, &bars[sl]);
+        auto cells = [&](unsigned char* to, const CUtensorMap* m) {
+            if constexpr (SKIP)
+                tma_load_3d(to, m, 4 * (x0 - 8), y0 - 8, z, &bars[sl]);
+            else
+                tma_load_4d(to, m, 0, x0 - 8, y0 - 8, z, &bars[sl]);
+        };
+        cells(dst + 2 * ADJ_F1, &tm.ma);
         if constexpr (TTI)
-            tma_load_4d(dst + 2 * ADJ_F1 + ADJ_F4, &tm.mb, 0, x0 - 8, y0 - 8, z, &bars[sl]);
+            cells(dst + 2 * ADJ_F1 + ADJ_F4, &tm.mb);
         else
             tma_load_3d(dst + 2 * ADJ_F1 + ADJ_F4, &tm.mb, x0 - 8, y0 - 8, z, &bars[sl]);
     };
@@ -801,6 +813,8 @@ __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__
             issue(t + ADJ_PF);
         }
         const int Lz = zs - LAG + t;
+        const bool inplane = !SKIP || (Lz >= zs && Lz <= ze);  // feeds x, y, xy of its own output
+        const bool mixed = TTI && (!SKIP || (Lz >= zs - kRadius && Lz <= ze + kRadius));  // feeds yz, zx of an output
         // point-wise values of the output plane L-7, loaded ahead of their use
         const int zo = Lz - LAG;
         const bool out_here = (zo >= zs) && owner;
@@ -848,18 +862,20 @@ __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__
             const float4 g = geo(k);
             irc = g.x;
             const float2 rho = f2(rcp_approx(g.x));
-            txx[ty * PW + tx + 8] = mul2(rho, fma2(f2(g.y * g.y), H, S));
-            tyy[(ty + 8) * TX + tx] = mul2(rho, fma2(f2(g.z * g.z), H, S));
             tz = mul2(rho, fma2(f2(g.w * g.w), H, S));
-            if constexpr (TTI) {
-                txy[(ty + 4) * IW + tx + 4] = mul2(f2(2.0f * g.y * g.z), H);
+            if (inplane) {
+                txx[ty * PW + tx + 8] = mul2(rho, fma2(f2(g.y * g.y), H, S));
+                tyy[(ty + 8) * TX + tx] = mul2(rho, fma2(f2(g.z * g.z), H, S));
+                if constexpr (TTI) txy[(ty + 4) * IW + tx + 4] = mul2(f2(2.0f * g.y * g.z), H);
+            }
+            if (mixed) {
                 tyz[(ty + 4) * TX + tx] = mul2(f2(2.0f * g.z * g.w), H);
                 tzx[ty * IW + tx + 4] = mul2(f2(2.0f * g.w * g.y), H);
             }
         }
         // rows above and below the core, columns 8..39: yy (rows 0..3, 28..31),
         // yy + xy + yz (rows 4..7, 24..27); one row per warp
-        {
+        if (inplane || (mixed && warp >= 8)) {
             const bool inner = warp >= 8;  // rows 4..7, 24..27
             const int w = warp & 7;
             const int r = inner ? (w < 4 ? 4 + w : 20 + w) : (w < 4 ? w : 24 + w);
@@ -880,7 +896,7 @@ __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__
         // 44..47; warps 0..3), xx + xy + zx (columns 4..7, 40..43; warps
         // 4..7); the xy corners (rows 4..7, 24..27 x columns 4..7, 40..43;
         // warps 8, 9)
-        if (warp < 8) {
+        if (warp < 8 && (inplane || (mixed && warp >= 4))) {
             const bool inner = warp >= 4;
             const int r = 8 + 4 * (warp & 3) + (lane >> 3), cc = lane & 7;
             const int c = inner ? (cc < 4 ? 4 + cc : 36 + cc) : (cc < 4 ? cc : 40 + cc);
@@ -895,7 +911,7 @@ __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__
                     tzx[(r - 8) * IW + c - 4] = mul2(f2(2.0f * g.w * g.y), H);
                 }
             }
-        } else if (TTI && warp < 10) {
+        } else if (TTI && inplane && warp >= 8 && warp < 10) {
             const int i = (warp - 8) * 32 + lane, rr = i >> 3, cc = i & 7;
             const int r = rr < 4 ? 4 + rr : 20 + rr, c = cc < 4 ? 4 + cc : 36 + cc;
             const int k = r * PW + c;
@@ -930,9 +946,12 @@ __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__
             for (int i = 1; i <= 4; ++i) acc = fma2(a.kd[1][i - 1], sub2(T[(i - 1) * TX], T[-i * TX]), acc);
             dys[r * TX + c] = in ? mul2(acc, f2(irv)) : f2(0.0f);
         };
-        dx_at(ty, tx + 4, irc);
-        dy_at(ty + 4, tx, irc);
-        if (warp < 4) {  // x halo of dxs: columns 0..3, 36..39
+        if (inplane) {
+            dx_at(ty, tx + 4, irc);
+            dy_at(ty + 4, tx, irc);
+        }
+        if (!inplane) {
+        } else if (warp < 4) {  // x halo of dxs: columns 0..3, 36..39
             const int i = warp * 32 + lane, r = i >> 3, cc = i & 7;
             const int c = cc < 4 ? cc : 32 + cc;
             dx_at(r, c, geo((r + 8) * PW + c + 4).x);
@@ -959,7 +978,7 @@ __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__
         // (4) yz/zx rhs: scatter of plane L into outputs L-4 .. L+4; output
         //     L-4 is then complete and moves to the in-plane queue
         float2 xy34 = f2(0.0f);
-        if constexpr (TTI) {
+        if (mixed) {
             // differences around this column, once per distance i: plane L
             // adds c2(i)*(T[+i] - T[-i]) to output L-i and its negative to L+i
             float2 dyz[4], dzx[4];
@@ -981,6 +1000,8 @@ __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__
 #pragma unroll
             for (int j = 0; j < 7; ++j) mq[j] = mq[j + 1];
             mq[7] = top;
+        }
+        if (TTI && inplane) {
             // xy of output L from plane L
             const int cc = tx + 4, rr = ty + 4;
 #pragma unroll
@@ -990,10 +1011,13 @@ __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__
                 xy34 = fma2(a.kxy[k - 1], sub2(add2(sub2(pp, pm), mm), mp), xy34);
             }
         }
-        __syncthreads();  // dxs/dys of plane L are ready
+        // dxs/dys of plane L are ready (a skipping plane that read nothing from
+        // the tiles leaves them to the next without a barrier)
+        if (inplane || mixed) __syncthreads();
 
         // (5) x+y parts of output L (dfdx_stg_right, kernel_type2_adj.cu:85-98)
-        {
+        sxy[7] = f2(0.0f);
+        if (inplane) {
             float2 acc = xy34;
 #pragma unroll
             for (int k = 1; k <= 4; ++k) {
@@ -1115,7 +1139,7 @@ __host__ __device__ constexpr size_t img_smem(size_t elt, bool tti)
 struct ImgMaps {
     CUtensorMap snap;   // 4D over the store: (nx, ny, nz, 4*nsnap), box PW x PH
     CUtensorMap p, q;   // adjoint p, q: box IW x IH
-    CUtensorMap ma;     // 4D (4, x, y, z), box 4 x IW x IH
+    CUtensorMap ma;     // float4 cells, box IW x IH
     CUtensorMap mb;     // TTI: like ma; VTI: irho, box IW x IH
     CUtensorMap snapc;  // the store again, box TX x TY
     CUtensorMap f3, f4; // adjoint pdot, qdot: box TX x TY
@@ -1195,9 +1219,9 @@ __global__ void __launch_bounds__(NT, 1) k_fused_image(const __grid_constant__ I
         unsigned char* adst = dst + 2 * IMG_P;
         tma_load_3d(adst, &tm.p, x0 - 4, y0 - 4, z, &bars[s]);
         tma_load_3d(adst + IMG_A, &tm.q, x0 - 4, y0 - 4, z, &bars[s]);
-        tma_load_4d(adst + 2 * IMG_A, &tm.ma, 0, x0 - 4, y0 - 4, z, &bars[s]);
+        tma_load_3d(adst + 2 * IMG_A, &tm.ma, 4 * (x0 - 4), y0 - 4, z, &bars[s]);
         if constexpr (TTI)
-            tma_load_4d(adst + 2 * IMG_A + IMG_A4, &tm.mb, 0, x0 - 4, y0 - 4, z, &bars[s]);
+            tma_load_3d(adst + 2 * IMG_A + IMG_A4, &tm.mb, 4 * (x0 - 4), y0 - 4, z, &bars[s]);
         else
             tma_load_3d(adst + 2 * IMG_A + IMG_A4, &tm.mb, x0 - 4, y0 - 4, z, &bars[s]);
         // point-wise values (zero-filled where z or z-LAG is outside the grid)
@@ -1259,12 +1283,8 @@ __global__ void __launch_bounds__(NT, 1) k_fused_image(const __grid_constant__ I
             pgv = CF[2 * TX * TY + kc0];
             pgr = CF[3 * TX * TY + kc0];
         }
-        const bool mirrored = a.fs && Lz < L.izbeg;
-        if (mirrored) {  // block-uniform
-            T* pt = reinterpret_cast<T*>(st);
-            for (int e = tid; e < 2 * PH * PW; e += NT) pt[e] = T(-to_f32(pt[e]));
-            __syncthreads();
-        }
+        const bool mirrored = a.fs && Lz < L.izbeg;  // such a plane is only read at its column
+        const bool inplane = Lz >= zs && Lz <= ze;   // the fill's planes feed z terms alone
         const T* P1 = reinterpret_cast<const T*>(st);
         const T* P2 = P1 + PH * PW;
         const float* AP = reinterpret_cast<const float*>(st + 2 * IMG_P);
@@ -1317,12 +1337,14 @@ __global__ void __launch_bounds__(NT, 1) k_fused_image(const __grid_constant__ I
             const float2 t2 = adj_t(k, g.x, g.z);
             ys[r * TX + c] = make_float4(acc.x, acc.y, t2.x, t2.y);
         };
-        xt_at(ty, tx);
-        // halos spread over warps 0..3 (x) and 4..11 (y): at most three
-        // tile cells per warp
-        if (tid < (IW - TX) * TY) xt_at(tid / (IW - TX), TX + tid % (IW - TX));
-        yt_at(ty, tx);
-        if (ty >= 4 && ty < 4 + IH - TY) yt_at(ty - 4 + TY, tx);
+        if (inplane) {
+            xt_at(ty, tx);
+            // halos spread over warps 0..3 (x) and 4..11 (y): at most three
+            // tile cells per warp
+            if (tid < (IW - TX) * TY) xt_at(tid / (IW - TX), TX + tid % (IW - TX));
+            yt_at(ty, tx);
+            if (ty >= 4 && ty < 4 + IH - TY) yt_at(ty - 4 + TY, tx);
+        }
         // (2) column values: z temporaries, buoyancy, D- z stage of the stored p/q
         {
             const float4 g = geo(kc);
@@ -1333,7 +1355,8 @@ __global__ void __launch_bounds__(NT, 1) k_fused_image(const __grid_constant__ I
 #pragma unroll
             for (int j = 0; j < 7; ++j) irq[j] = irq[j + 1];
             irq[7] = g.x;
-            const float2 v = spq((ty + 8) * PW + tx + 8);
+            const float2 v0 = spq((ty + 8) * PW + tx + 8);
+            const float2 v = mirrored ? make_float2(-v0.x, -v0.y) : v0;
 #pragma unroll
             for (int j = 0; j < 8; ++j) dzq[j] = fma2(f2(dminus_coef(j)), v, dzq[j]);
             const int zp = Lz - 3;
@@ -1355,7 +1378,10 @@ __global__ void __launch_bounds__(NT, 1) k_fused_image(const __grid_constant__ I
 
         // (3) x+y part of the gradient rhs at plane L (compute_xy_contributions
         //     of kernel_type2_grad.cu:314-342 and :435-439) and the Vp image
-        {
+#pragma unroll
+        for (int j = 0; j < 7; ++j) rxy[j] = rxy[j + 1];
+        rxy[7] = 0.0f;
+        if (inplane) {
             const int cx = ty * IW + tx + 4;    // x in the x-type tiles
             const int cy = (ty + 4) * TX + tx;  // y in the y-type tiles
             // positions -4 .. +4 around the cell, one 128-bit load each, folded
@@ -1393,8 +1419,6 @@ __global__ void __launch_bounds__(NT, 1) k_fused_image(const __grid_constant__ I
             v2 = fma2(make_float2(yc.z, yc.w), dfy, v2);
             v2 = fma2(dax, make_float2(xc.x, xc.y), v2);
             v2 = fma2(day, make_float2(yc.x, yc.y), v2);
-#pragma unroll
-            for (int j = 0; j < 7; ++j) rxy[j] = rxy[j + 1];
             rxy[7] = v2.x + v2.y;
             if (vp_here) a.gvp[dvp] = pgv + (pa3 * ps3 + pa4 * ps4);
         }
@@ -2045,27 +2069,45 @@ struct MapKey {
 std::mutex g_map_mu;
 std::map<MapKey, CUtensorMap> g_maps;
 
-// Map of a volume of float4 cells (the interleaved model), as a 4D tensor
-// (4, ldimx, ldimy, ldimz) with box (4, bx, by, 1): a tile lands in shared
-// memory as float4 [by][bx].
-bool make_map4(CUtensorMap* m, const float4* base, const Layout& L, int bx, int by)
+// Map of a volume of float4 cells (the interleaved model); a tile lands in
+// shared memory as float4 [by][bx].  rows: a 3D FP32 tensor (4*ldimx, ldimy,
+// ldimz) with box (4*bx, by, 1), copied in rows of 16*bx bytes; otherwise a 4D
+// tensor (4, ldimx, ldimy, ldimz) with box (4, bx, by, 1), copied cell by cell.
+// Rows arrive sooner (a 48x32 tile per plane and SM: 0.49 against 0.82 us) and
+// suit the kernels whose planes wait for them: imaging (256^3: 654 -> 626 us)
+// and the adjoint on short chunks, whose fill planes have little else to do
+// (101x93x77: 87 -> 73 us).  Under the full arithmetic of long chunks the
+// slower arrival costs nothing and disturbs the shared memory less (256^3
+// adjoint: 645 us by cells, 652 by rows).
+bool make_map4(CUtensorMap* m, const float4* base, const Layout& L, int bx, int by, bool rows)
 {
     auto fn = encode_fn();
-    if (!fn || !base) return false;
-    cuuint64_t dims[4] = {4, (cuuint64_t)L.ldimx, (cuuint64_t)L.ldimy, (cuuint64_t)L.ldimz};
-    cuuint64_t strides[3] = {(cuuint64_t)sizeof(float4), (cuuint64_t)L.ldimx * sizeof(float4),
-                             (cuuint64_t)L.ldimx * L.ldimy * sizeof(float4)};
-    cuuint32_t box[4] = {4, (cuuint32_t)bx, (cuuint32_t)by, 1};
+    if (!fn || !base || (rows && 4 * bx > 256)) return false;
+    const cuuint64_t row = (cuuint64_t)L.ldimx * sizeof(float4), plane = row * L.ldimy;
     cuuint32_t es[4] = {1, 1, 1, 1};
-    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float4*>(base), dims, strides, box, es,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUresult r;
+    if (rows) {
+        cuuint64_t dims[3] = {4 * (cuuint64_t)L.ldimx, (cuuint64_t)L.ldimy, (cuuint64_t)L.ldimz};
+        cuuint64_t strides[2] = {row, plane};
+        cuuint32_t box[3] = {4 * (cuuint32_t)bx, (cuuint32_t)by, 1};
+        r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float4*>(base), dims, strides, box, es,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    } else {
+        cuuint64_t dims[4] = {4, (cuuint64_t)L.ldimx, (cuuint64_t)L.ldimy, (cuuint64_t)L.ldimz};
+        cuuint64_t strides[3] = {(cuuint64_t)sizeof(float4), row, plane};
+        cuuint32_t box[4] = {4, (cuuint32_t)bx, (cuuint32_t)by, 1};
+        r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float4*>(base), dims, strides, box, es,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
     return r == CUDA_SUCCESS;
 }
 
-bool get_map4(CUtensorMap* out, const float4* p, const Layout& L, int bx, int by)
+bool get_map4(CUtensorMap* out, const float4* p, const Layout& L, int bx, int by, bool rows)
 {
-    MapKey k{reinterpret_cast<const float*>(p), -bx, by, L.ldimx, L.ldimy, L.ldimz};  // negative width: float4 cells
+    // negative sizes: float4 cells, by rows
+    MapKey k{reinterpret_cast<const float*>(p), -bx, rows ? -by : by, L.ldimx, L.ldimy, L.ldimz};
     std::lock_guard<std::mutex> lk(g_map_mu);
     auto it = g_maps.find(k);
     if (it != g_maps.end()) {
@@ -2073,7 +2115,7 @@ bool get_map4(CUtensorMap* out, const float4* p, const Layout& L, int bx, int by
         return true;
     }
     CUtensorMap m;
-    if (!make_map4(&m, p, L, bx, by)) return false;
+    if (!make_map4(&m, p, L, bx, by, rows)) return false;
     if (g_maps.size() > 4096) g_maps.clear();
     g_maps[k] = m;
     *out = m;
@@ -2129,7 +2171,9 @@ bool prepare_device()
 {
     bool ok = err_word() != nullptr;
     ok = ok && set_smem(k_fused_forward<false>, FWD_SMEM) && set_smem(k_fused_forward<true>, FWD_SMEM);
-    ok = ok && set_smem(k_fused_adjoint<false>, adj_smem(false)) && set_smem(k_fused_adjoint<true>, adj_smem(true));
+    ok = ok && set_smem(k_fused_adjoint<false, false>, adj_smem(false)) &&
+         set_smem(k_fused_adjoint<true, false>, adj_smem(true)) &&
+         set_smem(k_fused_adjoint<false, true>, adj_smem(false)) && set_smem(k_fused_adjoint<true, true>, adj_smem(true));
     ok = ok && set_smem(k_fused_image<false, float>, img_smem(4, false)) &&
          set_smem(k_fused_image<true, float>, img_smem(4, true));
     ok = ok && set_smem(k_fused_image<false, __half>, img_smem(2, false)) &&
@@ -2230,10 +2274,20 @@ std::vector<int> plane_candidates(const Layout& L)
 int kind_ctas_per_sm(int kind) { return kind == KIND_T1F ? 2 : 1; }
 
 // Modelled time of a step, in plane-iterations of the slowest CTA: per_sm
-// resident CTAs per SM, each segment pays the 2*LAG-plane pipeline fill, a
-// range of bz planes covers at most ceil((bz-1)/nz)+1 columns (one when
-// whole columns divide evenly).
-double plane_cost(const Layout& L, int bz, int lag, int per_sm)
+// resident CTAs per SM, each segment pays the 2*lag-plane pipeline fill
+// (weighed, see fill_weight), a range of bz planes covers at most
+// ceil((bz-1)/nz)+1 columns (one when whole columns divide evenly).
+//
+// A fill plane counts fill_weight of an output's plane: it has no output
+// stage, in the forward kernel (which does its in-plane work there) hardly more
+// than the mixed terms, and the imaging and short-chunk adjoint kernels skip
+// most of it.  With these weights the model chooses what the autotuner does at
+// 256^3 (adjoint and imaging 148/233, forward 199/225; a weight of 1 gave
+// 96/241, 2 % slower), 224x224x160 (forward 104/107, 2 %) and 101x93x77
+// (forward 13/14: 62 us against 73 us with 11/22).
+double fill_weight(int kind) { return kind == KIND_FWD ? 0.3 : 0.55; }
+
+double plane_cost(const Layout& L, int bz, double lag, int per_sm)
 {
     const int nz = L.nz();
     const long long ctas = cta_count(L, Split{bz, 0});
@@ -2254,14 +2308,18 @@ double plane_cost(const Layout& L, int bz, int lag, int per_sm)
 // that neighbouring tiles share are still in L2 when the neighbour reads
 // them.  Unaligned shares balance the SMs better but spread the CTAs over
 // all of z; a kernel that stages many halo'd arrays then re-reads its halos
-// from HBM (the adjoint stages nine, the imaging kernel eleven; the forward
-// kernel three).
+// from HBM (the adjoint stages nine, the imaging kernel eleven).  The forward
+// kernels stage three and two: an unaligned share counts 1.2 times its
+// modelled cost for them.  512x512x400: 2.47 ms in aligned shares of 200
+// planes, 2.96 ms in unaligned ones of 1384, which the model alone puts 3 %
+// below; 256^3: 611 us top/bottom (199/225), 607 us in unaligned shares of
+// 222 planes with twice the DRAM bytes.
 bool column_aligned(const Layout& L, int bz) { return bz <= L.nz() && L.nz() % bz == 0; }
 
 // Modelled cost of a top/bottom split in one wave: the tops (one segment
 // each) against the bottom CTAs, whose bz planes cross at most
 // ceil((bz-1)/span)+1 column bottoms.
-double split_cost(const Layout& L, Split sp, int lag, int per_sm)
+double split_cost(const Layout& L, Split sp, double lag, int per_sm)
 {
     const int span = L.nz() - sp.ztop;
     const int segs = (sp.bz - 1) / span + 2;
@@ -2299,16 +2357,19 @@ std::vector<Split> topbottom_candidates(const Layout& L, int kind)
 }
 
 // The model's split: the cheapest tile-major candidate (column-aligned only
-// for the kernels that stage many halo'd arrays) or top/bottom split.
+// for the kernels that stage many halo'd arrays, at a handicap for the others
+// when it is not) or top/bottom split.
 Split pick_split(const Layout& L, int kind)
 {
     Split best{L.nz(), 0};
     double best_cost = 1e300;
     const bool any_split = kind == KIND_FWD || kind == KIND_T1F;  // few staged arrays
-    const int lag = kind_lag(kind), per_sm = kind_ctas_per_sm(kind);
+    const double lag = fill_weight(kind) * kind_lag(kind);
+    const int per_sm = kind_ctas_per_sm(kind);
     for (int bz : plane_candidates(L)) {
-        if (!any_split && !column_aligned(L, bz)) continue;
-        const double cost = plane_cost(L, bz, lag, per_sm);
+        const bool aligned = column_aligned(L, bz);
+        if (!any_split && !aligned) continue;
+        const double cost = plane_cost(L, bz, lag, per_sm) * (aligned ? 1.0 : 1.2);
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = Split{bz, 0};
@@ -2387,16 +2448,29 @@ int launch_fused_forward(const Layout& L, const FwdStepArgs& s, cudaStream_t st)
     return launch_status();
 }
 
+namespace {
+// Whether the adjoint kernel skips the work that the pipeline fill's planes
+// do for nobody: where a CTA's segments are of at most 64 planes (a column
+// top's when the split has tops), the fill being 18 % of the planes and more.
+// Measured with and without: 48x40x40 TTI (2-plane chunks) 27 / 41 us, 101x93x77
+// TTI (14) 73 / 97, 96^3 VTI (12) 40 / 50, 128^3 VTI (32) 79 / 86, 224x224x160
+// VTI (115) 238 / 234, 256^3 TTI (241) 699 / 665.
+bool adj_skips_fill(const Layout& L, Split sp) { return std::min(L.nz(), sp.ztop > 0 ? sp.ztop : sp.bz) <= 64; }
+} // namespace
+
 int launch_fused_adjoint(const Layout& L, const AdjStepArgs& s, cudaStream_t st)
 {
     if (!layout_supported(L)) return TTI_EINVAL;
     const bool tti = !s.vti;
     if (!s.m.ma || (tti && !s.m.mb)) return TTI_EINVAL;
+    const Split sp = s.bz > 0 ? Split{s.bz, s.ztop} : choose_split(L, KIND_ADJ);
+    if (!split_valid(L, sp)) return TTI_EINVAL;
+    const bool skip = adj_skips_fill(L, sp);
     AdjMaps tm;
     if (!get_map(&tm.p, s.pin, L, PW, PH) || !get_map(&tm.q, s.qin, L, PW, PH) ||
-        !get_map4(&tm.ma, s.m.ma, L, PW, PH))
+        !get_map4(&tm.ma, s.m.ma, L, PW, PH, skip))
         return TTI_ELAUNCH;
-    if (tti ? !get_map4(&tm.mb, s.m.mb, L, PW, PH) : !get_map(&tm.mb, s.m.irho, L, PW, PH)) return TTI_ELAUNCH;
+    if (tti ? !get_map4(&tm.mb, s.m.mb, L, PW, PH, skip) : !get_map(&tm.mb, s.m.irho, L, PW, PH)) return TTI_ELAUNCH;
     AdjParams a{};
     a.pout = s.pout;
     a.qout = s.qout;
@@ -2408,8 +2482,6 @@ int launch_fused_adjoint(const Layout& L, const AdjStepArgs& s, cudaStream_t st)
     a.aby = s.aby;
     a.abz = s.abz;
     a.L = L;
-    const Split sp = s.bz > 0 ? Split{s.bz, s.ztop} : choose_split(L, KIND_ADJ);
-    if (!split_valid(L, sp)) return TTI_EINVAL;
     a.bz = sp.bz;
     a.ztop = sp.ztop;
     a.fs = s.free_surface;
@@ -2440,10 +2512,15 @@ int launch_fused_adjoint(const Layout& L, const AdjStepArgs& s, cudaStream_t st)
     if (!a.err) return TTI_ENOMEM;
     dim3 grid(cta_count(L, sp));
     if (!kernels_prepared()) return TTI_ELAUNCH;
-    if (!tti)
-        k_fused_adjoint<false><<<grid, dim3(TX, TY), adj_smem(false), st>>>(tm, a);
+    const dim3 block(TX, TY);
+    if (!tti && skip)
+        k_fused_adjoint<false, true><<<grid, block, adj_smem(false), st>>>(tm, a);
+    else if (!tti)
+        k_fused_adjoint<false, false><<<grid, block, adj_smem(false), st>>>(tm, a);
+    else if (skip)
+        k_fused_adjoint<true, true><<<grid, block, adj_smem(true), st>>>(tm, a);
     else
-        k_fused_adjoint<true><<<grid, dim3(TX, TY), adj_smem(true), st>>>(tm, a);
+        k_fused_adjoint<true, false><<<grid, block, adj_smem(true), st>>>(tm, a);
     return launch_status();
 }
 
@@ -2502,9 +2579,9 @@ int launch_fused_image(const Layout& L, const ImageArgs& s, cudaStream_t st)
     const bool tti = !s.vti;
     if (!s.m.ma || (tti && !s.m.mb)) return TTI_EINVAL;
     if (!get_map(&tm.p, s.adj1, L, IW, IH) || !get_map(&tm.q, s.adj2, L, IW, IH) ||
-        !get_map4(&tm.ma, s.m.ma, L, IW, IH))
+        !get_map4(&tm.ma, s.m.ma, L, IW, IH, true))
         return TTI_ELAUNCH;
-    if (tti ? !get_map4(&tm.mb, s.m.mb, L, IW, IH) : !get_map(&tm.mb, s.m.irho, L, IW, IH)) return TTI_ELAUNCH;
+    if (tti ? !get_map4(&tm.mb, s.m.mb, L, IW, IH, true) : !get_map(&tm.mb, s.m.irho, L, IW, IH)) return TTI_ELAUNCH;
     if (!get_map(&tm.f3, s.adj3, L, TX, TY) || !get_map(&tm.f4, s.adj4, L, TX, TY)) return TTI_ELAUNCH;
     if (!make_store_map(&tm.snapc, s.store, s.snap_prec, L.nx(), L.ny(), L.nz(), 4 * s.nsnap, TX, TY) ||
         !make_store_map(&tm.gv, s.grad_vp, SNAP_F32, L.nx(), L.ny(), L.nz(), 1, TX, TY) ||
