@@ -51,6 +51,13 @@ int launch_rho_gradient_with_base(float* grad, const float* fd1x, const float* f
                                   int ixend, int iybeg, int iyend, int izbeg, int izend, int ldimx, int ldimy,
                                   int gldx, int gldy, double dx, double dy, double dz, cudaStream_t st);
 
+// tti_launch_type1_adj on a caller's scratch of float4 cells.
+int launch_t1_adj_with_base(float* f3, float* f4, const float* f1, const float* f2, const float* m1, const float* m2,
+                            const float* m3, const float* m4, const float* rx, const float* ry, const float* rz,
+                            const float* abx, const float* aby, const float* abz, float4* base, int ixbeg, int ixend,
+                            int iybeg, int iyend, int izbeg, int izend, int ldimx, int ldimy, float dt, double dx,
+                            double dy, double dz, int use_sponge, cudaStream_t st);
+
 // Receiver cells for the step kernels: the receivers lie on nz planes with
 // halo'd z index z[k]; plane k's table of receiver numbers per interior cell
 // (-1: none) starts at off[k] in xy.  Passed by value, so the plane check of

@@ -540,17 +540,28 @@ int forward_per_kernel_step(tti_sim* s, int n, cudaStream_t st)
     return launch_status();
 }
 
+// The centred launcher sequence's adjoint scratch (the launcher allocates its
+// own per call): taken when an adjoint pass begins, outside any capture, and
+// kept with the simulator.  Taken and given back per call it is mapped afresh
+// around every synchronizing adjoint(): 150x141x133, 16 steps, 7.1 ms a shot
+// against 5.3.
+int ensure_t1_scratch(tti_sim* s)
+{
+    if (s->cfg.scheme != 1 || s->cfg.fused || s->base) return TTI_OK;
+    return s->alloc((void**)&s->base, (size_t)s->nvol() * sizeof(float4));
+}
+
 int adjoint_per_kernel_step(tti_sim* s, cudaStream_t st)
 {
     const Layout& L = s->L;
     const tti_sim_config& c = s->cfg;
     WaveState& w = s->w;
     if (c.scheme == 1) {  // kernels/kernel_type1_gpu_adj.cu, then loop2 and loop4
-        int rc = tti_launch_type1_adj(w.pd, w.qd, w.p, w.q, s->mv[1], s->mv[2], s->mv[3], s->mv[4], s->mv[5],
-                                      s->mv[6], s->mv[7], (const float*)s->abx, (const float*)s->aby,
-                                      (const float*)s->abz, L.ixbeg, L.ixend, L.iybeg, L.iyend, L.izbeg, L.izend,
-                                      L.ldimx, L.ldimy, L.ldimz, c.dt, c.dx, c.dy, c.dz, 8, st,
-                                      s->sponge_active ? 1 : 0, 0);
+        int rc = launch_t1_adj_with_base(w.pd, w.qd, w.p, w.q, s->mv[1], s->mv[2], s->mv[3], s->mv[4], s->mv[5],
+                                         s->mv[6], s->mv[7], (const float*)s->abx, (const float*)s->aby,
+                                         (const float*)s->abz, s->base, L.ixbeg, L.ixend, L.iybeg, L.iyend, L.izbeg,
+                                         L.izend, L.ldimx, L.ldimy, c.dt, c.dx, c.dy, c.dz, s->sponge_active ? 1 : 0,
+                                         st);
         if (rc) return rc;
         s->launches += 2;
         if ((rc = tti_launch_kernel_loop2(w.p, w.q, w.pd, w.qd, L.ldimx, L.ldimy, L.ixbeg, L.ixend, L.iybeg,
@@ -1274,7 +1285,8 @@ static int sim_adjoint(tti_sim* s, const float* residual, int residual_on_device
     cudaStream_t st0 = s->stream;
     s->launches = 0;
     s->st_mode = 0;
-    int rc = zero_state(s, s->w);
+    int rc = ensure_t1_scratch(s);
+    if (!rc) rc = zero_state(s, s->w);
     if (!rc) rc = sim_zero(s, s->grad_vp, s->ninterior * sizeof(float));
     if (!rc) rc = sim_zero(s, s->grad_rho, s->ninterior * sizeof(float));
     if (rc) return rc;
@@ -1396,7 +1408,8 @@ int tti_sim_adjoint_begin(tti_sim* s, const float* residual, int residual_on_dev
     const tti_sim_config& c = s->cfg;
     s->launches = 0;
     s->st_mode = 0;
-    int rc = zero_state(s, s->w);
+    int rc = ensure_t1_scratch(s);
+    if (!rc) rc = zero_state(s, s->w);
     if (!rc) rc = sim_zero(s, s->grad_vp, s->ninterior * sizeof(float));
     if (!rc) rc = sim_zero(s, s->grad_rho, s->ninterior * sizeof(float));
     if (!rc && s->nrec) {
