@@ -30,7 +30,7 @@ namespace {
 
 constexpr int E3X = 32, E3Y = 8;  // threads per block: one warp row per y
 constexpr int E3Z = 16;           // planes per thread (point-wise kernels)
-constexpr int E3ZC = 64;          // planes per thread (z-windowed velocity kernels)
+constexpr int E3ZC = 64;          // most planes per thread (z-windowed velocity kernels)
 
 __device__ __forceinline__ float e3_df(int i)
 {
@@ -47,6 +47,18 @@ struct E3Grid {
     int nx, ny, nz, ldimx, ldimy;
     __device__ int64_t idx(int ix, int iy, int iz) const { return ((int64_t)iz * ldimy + iy) * ldimx + ix; }
 };
+
+// Planes per block of the z-windowed kernels: the most that leaves six blocks
+// for each of the 148 SMs, 16 at least (a chunk starts with eight planes of
+// window loads).  211x187x150 (504 blocks of 64 planes): velocity update 135 -> 107 us,
+// strains 97 -> 79 us.
+int e3_zchunk(const E3Grid& g)
+{
+    const int64_t columns = (int64_t)((g.nx + E3X - 1) / E3X) * ((g.ny + E3Y - 1) / E3Y);
+    int zper = E3ZC;
+    while (zper > 16 && columns * ((g.nz + zper - 1) / zper) < 6 * 148) zper /= 2;
+    return zper;
+}
 
 dim3 e3_blocks(const E3Grid& g, int zper) { return dim3((g.nx + E3X - 1) / E3X, (g.ny + E3Y - 1) / E3Y, (g.nz + zper - 1) / zper); }
 
@@ -116,7 +128,7 @@ __global__ void __launch_bounds__(E3X* E3Y) k_e3_vgplain(const float* __restrict
                                                         float* __restrict__ d5, float* __restrict__ d6,
                                                         float* __restrict__ d7, float* __restrict__ d8,
                                                         float* __restrict__ d9, const float* __restrict__ zprime,
-                                                        E3Grid g)
+                                                        E3Grid g, int zper)
 {
     __shared__ __align__(16) float t1[2][E3Y + 8][E3X + 8], t2[2][E3Y + 8][E3X + 8], t3[2][E3Y + 8][E3X + 8];
     __shared__ __align__(16) float tw[2][3][E3Y][E3X];  // f1, f2, f3 of plane iz+4 (the windows' new plane)
@@ -126,7 +138,7 @@ __global__ void __launch_bounds__(E3X* E3Y) k_e3_vgplain(const float* __restrict
     const bool act = ix < 4 + g.nx && iy < 4 + g.ny;
     const float invd1 = 1.01f, invd2 = 2.02f;
     const int64_t sz = (int64_t)g.ldimx * g.ldimy;
-    const int z0 = 4 + blockIdx.z * E3ZC, z1 = min(z0 + E3ZC, 4 + g.nz);
+    const int z0 = 4 + blockIdx.z * zper, z1 = min(z0 + zper, 4 + g.nz);
     float w1[9] = {}, w2[9] = {}, w3[9] = {};  // planes iz-4 .. iz+4
     if (act) {
         const int64_t i0 = g.idx(ix, iy, z0 - 4);
@@ -188,28 +200,38 @@ __global__ void __launch_bounds__(E3X* E3Y) k_e3_vgplain(const float* __restrict
 // -- except that planes s <= 6, which the reference adds while priming its
 // queues, weigh by INT_S_O8[max(3 - s, s - 4)] (its loop at :120-129 uses
 // the arriving plane's index): the blocking shows in its result, and it is
-// kept.  Slot 0 is complete once its eighth plane has arrived.  The planes
-// come through double-buffered shared tiles with a halo of 4.
+// kept.  Slot 0 is complete once its eighth plane has arrived.
+// The two pairs of a plane that feed slots i and 7 - i are the same cells.
+//
+// All six precomputes are one launch (blockIdx.z = volume x z block): six
+// launches of 1024 blocks each ended in a nearly empty SM, and each waits for
+// memory more than for bandwidth.  A thread owns two rows (8 apart) of a 32x16
+// tile, whose halo costs 1.9 loads per output instead of 2.5.  256^3: the six
+// 520 -> 468 us (12 B/pt each, 31 us at the copy rate; the waits remain).
+constexpr int E3PY = 2 * E3Y;
+
+struct E3Pre {
+    const float* in[6];
+    float *xz[6], *yz[6];
+};
+
 template <int XS, int YS, int ZS, int V>
-__global__ void __launch_bounds__(E3X* E3Y) k_e3_precompute(const float* __restrict__ in, float* __restrict__ xz,
-                                                           float* __restrict__ yz, E3Grid g)
+__device__ __forceinline__ void e3_precompute(float (&t)[3][E3PY + 8][E3X + 8], const float* __restrict__ in,
+                                              float* __restrict__ xz, float* __restrict__ yz, const E3Grid& g, int b)
 {
     // planes staged in triple-buffered shared tiles (halo 4) by async copies,
     // two planes in flight while one is used
-    __shared__ __align__(16) float t[3][E3Y + 8][E3X + 8];
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * E3X + tx;
-    const int x0 = 4 + blockIdx.x * E3X, y0 = 4 + blockIdx.y * E3Y;
-    const int ix = x0 + tx, iy = y0 + ty;
-    const bool act = ix < 4 + g.nx && iy < 4 + g.ny;
+    const int x0 = 4 + blockIdx.x * E3X, y0 = 4 + blockIdx.y * E3PY;
+    const int ix = x0 + tx;
     constexpr int X1 = -3 - XS, X2 = 4 - XS, Y1 = -3 - YS, Y2 = 4 - YS;
-    const int b = blockIdx.z;
     const int mend = min(64, g.nz - 64 * b), p0 = 64 * b + 1 - ZS;
     const int64_t sz = (int64_t)g.ldimx * g.ldimy;
-    float* oxz = xz + g.idx(ix, iy, 4 + 64 * b);
-    float* oyz = yz + g.idx(ix, iy, 4 + 64 * b);
-    float qxz[8], qyz[8];
+    float qxz[2][8], qyz[2][8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) qxz[i] = qyz[i] = 0.0f;
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) qxz[r][i] = qyz[r][i] = 0.0f;
     const int ns = mend + 7;
     auto stage = [&](int bb, int s) {
         stage_tile_async<V>(t[bb], in + (int64_t)(p0 + s) * sz, x0 - 4, y0 - 4, g, tid);
@@ -221,37 +243,54 @@ __global__ void __launch_bounds__(E3X* E3Y) k_e3_precompute(const float* __restr
         if (s + 2 < ns) stage(bb == 0 ? 2 : bb - 1, s + 2);  // the buffer plane s-1 used
         __pipeline_wait_prior(s + 2 < ns ? 2 : s + 1 < ns ? 1 : 0);
         __syncthreads();
-        const float* pl = &t[bb][ty + 4][tx + 4];
         constexpr int S = E3X + 8;
-        if (s <= 6) {  // priming: one weight for the whole plane
-            const int ic = max(3 - s, s - 4);
-            const float c = ic == 0 ? e3_int(0) : ic == 1 ? e3_int(1) : ic == 2 ? e3_int(2) : e3_int(3);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                qxz[i] += c * (pl[X1 + i] + pl[X2 - i]);
-                qyz[i] += c * (pl[(Y1 + i) * S] + pl[(Y2 - i) * S]);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float c = e3_int(max(3 - i, i - 4));
-                qxz[i] += c * (pl[X1 + i] + pl[X2 - i]);
-                qyz[i] += c * (pl[(Y1 + i) * S] + pl[(Y2 - i) * S]);
-            }
-        }
+        // priming (s <= 6): one weight for the whole plane
+        const int ic = max(3 - s, s - 4);
+        const float cp = ic == 0 ? e3_int(0) : ic == 1 ? e3_int(1) : ic == 2 ? e3_int(2) : e3_int(3);
         const int m = s - 7;  // the output slot 0 holds
-        if (act && m >= 0) {
-            oxz[m * sz] = 0.5f * qxz[0];
-            oyz[m * sz] = 0.5f * qyz[0];
-        }
 #pragma unroll
-        for (int i = 0; i < 7; ++i) {
-            qxz[i] = qxz[i + 1];
-            qyz[i] = qyz[i + 1];
+        for (int r = 0; r < 2; ++r) {
+            const float* pl = &t[bb][ty + r * E3Y + 4][tx + 4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float c = s <= 6 ? cp : e3_int(3 - i);
+                const float px = pl[X1 + i] + pl[X2 - i], py = pl[(Y1 + i) * S] + pl[(Y2 - i) * S];
+                qxz[r][i] += c * px;
+                qxz[r][7 - i] += c * px;
+                qyz[r][i] += c * py;
+                qyz[r][7 - i] += c * py;
+            }
+            const int iy = y0 + ty + r * E3Y;
+            if (m >= 0 && ix < 4 + g.nx && iy < 4 + g.ny) {
+                const int64_t o = g.idx(ix, iy, 4 + 64 * b + m);
+                xz[o] = 0.5f * qxz[r][0];
+                yz[o] = 0.5f * qyz[r][0];
+            }
+#pragma unroll
+            for (int i = 0; i < 7; ++i) {
+                qxz[r][i] = qxz[r][i + 1];
+                qyz[r][i] = qyz[r][i + 1];
+            }
+            qxz[r][7] = qyz[r][7] = 0.0f;
         }
-        qxz[7] = qyz[7] = 0.0f;
         __syncthreads();  // every thread is done with buffer bb before it is refilled
     }
+}
+
+// Volumes 0..2 (11, 22, 33) shift x, y and z; 3 (12) z; 4 (13) y; 5 (23) x.
+template <int V>
+__global__ void __launch_bounds__(E3X* E3Y) k_e3_precompute(E3Pre a, E3Grid g)
+{
+    __shared__ __align__(16) float t[3][E3PY + 8][E3X + 8];
+    const int v = blockIdx.z % 6, b = blockIdx.z / 6;
+    if (v < 3)
+        e3_precompute<1, 1, 1, V>(t, a.in[v], a.xz[v], a.yz[v], g, b);
+    else if (v == 3)
+        e3_precompute<0, 0, 1, V>(t, a.in[3], a.xz[3], a.yz[3], g, b);
+    else if (v == 4)
+        e3_precompute<0, 1, 0, V>(t, a.in[4], a.xz[4], a.yz[4], g, b);
+    else
+        e3_precompute<1, 0, 0, V>(t, a.in[5], a.xz[5], a.yz[5], g, b);
 }
 
 struct E3Stress {
@@ -362,7 +401,7 @@ __global__ void __launch_bounds__(E3X* E3Y) k_e3_vplain(float* __restrict__ f1, 
                                                        const float* __restrict__ f5, const float* __restrict__ f6,
                                                        const float* __restrict__ f7, const float* __restrict__ f8,
                                                        const float* __restrict__ f9, const float* __restrict__ M22,
-                                                       const float* __restrict__ zprime, E3Grid g)
+                                                       const float* __restrict__ zprime, E3Grid g, int zper)
 {
     __shared__ __align__(16) float t4[2][E3Y][E3X + 8], t8[2][E3Y][E3X + 8];  // x taps
     __shared__ __align__(16) float t5[2][E3Y + 8][E3X], t9[2][E3Y + 8][E3X];  // y taps
@@ -376,7 +415,7 @@ __global__ void __launch_bounds__(E3X* E3Y) k_e3_vplain(float* __restrict__ f1, 
     const bool act = ix < 4 + g.nx && iy < 4 + g.ny;
     const float invd1 = 1.01f, invd2 = 2.01f;
     const int64_t sz = (int64_t)g.ldimx * g.ldimy;
-    const int z0 = 4 + blockIdx.z * E3ZC, z1 = min(z0 + E3ZC, 4 + g.nz);
+    const int z0 = 4 + blockIdx.z * zper, z1 = min(z0 + zper, 4 + g.nz);
     float w6[9] = {}, w8[9] = {}, w9[9] = {};  // planes iz-4 .. iz+4
     float m22z = 0.0f;
     if (act) {
@@ -537,12 +576,13 @@ int tti_e3_launch_vgplain(const float* f1, const float* f2, const float* f3, flo
         !zprime)
         return TTI_EINVAL;
     const E3Grid g{nx, ny, nz, ldimx, ldimy};
+    const int zper = e3_zchunk(g);
     if (vec4_ok(ldimx, {f1, f2, f3}))
-        k_e3_vgplain<4><<<e3_blocks(g, E3ZC), dim3(E3X, E3Y), 0, S(stream)>>>(f1, f2, f3, d4, d5, d6, d7, d8, d9,
-                                                                              zprime, g);
+        k_e3_vgplain<4><<<e3_blocks(g, zper), dim3(E3X, E3Y), 0, S(stream)>>>(f1, f2, f3, d4, d5, d6, d7, d8, d9,
+                                                                              zprime, g, zper);
     else
-        k_e3_vgplain<1><<<e3_blocks(g, E3ZC), dim3(E3X, E3Y), 0, S(stream)>>>(f1, f2, f3, d4, d5, d6, d7, d8, d9,
-                                                                              zprime, g);
+        k_e3_vgplain<1><<<e3_blocks(g, zper), dim3(E3X, E3Y), 0, S(stream)>>>(f1, f2, f3, d4, d5, d6, d7, d8, d9,
+                                                                              zprime, g, zper);
     return launch_status();
 }
 
@@ -561,23 +601,14 @@ int tti_e3_launch_splain(float* f4, float* f5, float* f6, float* f7, float* f8, 
     const E3Grid g{nx, ny, nz, ldimx, ldimy};
     cudaStream_t st = S(stream);
     // the six z-mixed precomputes of sPlainLoop (simulator3SetUp.cu:1177-1186)
-    const dim3 pb((nx + E3X - 1) / E3X, (ny + E3Y - 1) / E3Y, (nz - 1) / 64 + 1), t(E3X, E3Y);
+    const dim3 pb((nx + E3X - 1) / E3X, (ny + E3PY - 1) / E3PY, 6 * ((nz - 1) / 64 + 1)), t(E3X, E3Y);
     float* const* p = f10_21;
-    if (vec4_ok(ldimx, {f1_1, f2_2, f3_3, f1_2, f1_3, f2_3})) {
-        k_e3_precompute<1, 1, 1, 4><<<pb, t, 0, st>>>(f1_1, p[0], p[1], g);
-        k_e3_precompute<1, 1, 1, 4><<<pb, t, 0, st>>>(f2_2, p[6], p[7], g);
-        k_e3_precompute<1, 1, 1, 4><<<pb, t, 0, st>>>(f3_3, p[10], p[11], g);
-        k_e3_precompute<0, 0, 1, 4><<<pb, t, 0, st>>>(f1_2, p[2], p[3], g);
-        k_e3_precompute<0, 1, 0, 4><<<pb, t, 0, st>>>(f1_3, p[4], p[5], g);
-        k_e3_precompute<1, 0, 0, 4><<<pb, t, 0, st>>>(f2_3, p[8], p[9], g);
-    } else {
-        k_e3_precompute<1, 1, 1, 1><<<pb, t, 0, st>>>(f1_1, p[0], p[1], g);
-        k_e3_precompute<1, 1, 1, 1><<<pb, t, 0, st>>>(f2_2, p[6], p[7], g);
-        k_e3_precompute<1, 1, 1, 1><<<pb, t, 0, st>>>(f3_3, p[10], p[11], g);
-        k_e3_precompute<0, 0, 1, 1><<<pb, t, 0, st>>>(f1_2, p[2], p[3], g);
-        k_e3_precompute<0, 1, 0, 1><<<pb, t, 0, st>>>(f1_3, p[4], p[5], g);
-        k_e3_precompute<1, 0, 0, 1><<<pb, t, 0, st>>>(f2_3, p[8], p[9], g);
-    }
+    const E3Pre pre{{f1_1, f2_2, f3_3, f1_2, f1_3, f2_3}, {p[0], p[6], p[10], p[2], p[4], p[8]},
+                    {p[1], p[7], p[11], p[3], p[5], p[9]}};
+    if (vec4_ok(ldimx, {f1_1, f2_2, f3_3, f1_2, f1_3, f2_3}))
+        k_e3_precompute<4><<<pb, t, 0, st>>>(pre, g);
+    else
+        k_e3_precompute<1><<<pb, t, 0, st>>>(pre, g);
     E3Stress a{};
     float* out[6] = {f4, f5, f6, f7, f8, f9};
     a.f4 = out[0];
@@ -618,12 +649,13 @@ int tti_e3_launch_vplain(float* f1, float* f2, float* f3, const float* f4, const
         !M22 || !zprime)
         return TTI_EINVAL;
     const E3Grid g{nx, ny, nz, ldimx, ldimy};
+    const int zper = e3_zchunk(g);
     if (vec4_ok(ldimx, {f1, f2, f3, f4, f5, f6, f7, f8, f9, M22}))
-        k_e3_vplain<4><<<e3_blocks(g, E3ZC), dim3(E3X, E3Y), 0, S(stream)>>>(f1, f2, f3, f4, f5, f6, f7, f8, f9, M22,
-                                                                             zprime, g);
+        k_e3_vplain<4><<<e3_blocks(g, zper), dim3(E3X, E3Y), 0, S(stream)>>>(f1, f2, f3, f4, f5, f6, f7, f8, f9, M22,
+                                                                             zprime, g, zper);
     else
-        k_e3_vplain<1><<<e3_blocks(g, E3ZC), dim3(E3X, E3Y), 0, S(stream)>>>(f1, f2, f3, f4, f5, f6, f7, f8, f9, M22,
-                                                                             zprime, g);
+        k_e3_vplain<1><<<e3_blocks(g, zper), dim3(E3X, E3Y), 0, S(stream)>>>(f1, f2, f3, f4, f5, f6, f7, f8, f9, M22,
+                                                                             zprime, g, zper);
     return launch_status();
 }
 
