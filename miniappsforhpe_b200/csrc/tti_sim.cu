@@ -350,6 +350,7 @@ struct Plan {
     size_t core = 0, aux = 0, snaps = 0, ckpts = 0, recompute = 0;
     bool need_aux = false;
     bool packed_model = false;  // interleaved model volumes for the fused staggered adjoint
+    bool t1_scratch = false;    // the centred launcher sequence's adjoint scratch
     int nsnap = 0, nslot = 0, ncp = 0;
     size_t total() const { return core + aux + snaps + ckpts + recompute; }
 };
@@ -369,6 +370,11 @@ Plan plan_of(const tti_sim_config& c)
     // derivative volumes and scratch: only the staggered scheme's kernel sequence
     pl.need_aux = c.scheme == 0 && (!c.fused || (c.save_snapshots && !fused_image_supported(L)));
     if (pl.need_aux) pl.aux = 10 * vb + 4 * vb;  // rhs3, rhs4, snp, snq, six derivatives, 4-float scratch
+    // The centred launcher sequence's adjoint works in a scratch of float4
+    // cells (the launcher by itself allocates one per call; taken and given
+    // back per call it is mapped afresh around every synchronizing adjoint()).
+    pl.t1_scratch = c.scheme == 1 && !c.fused && c.save_snapshots;
+    if (pl.t1_scratch) pl.aux = 4 * vb;
     if (c.save_snapshots) {
         pl.nsnap = (c.nt - 1) / c.xcorr_step + 1;
         pl.nslot = pl.nsnap;
@@ -556,17 +562,6 @@ int forward_per_kernel_step(tti_sim* s, int n, cudaStream_t st)
         s->launches++;
     }
     return launch_status();
-}
-
-// The centred launcher sequence's adjoint scratch (the launcher allocates its
-// own per call): taken when an adjoint pass begins, outside any capture, and
-// kept with the simulator.  Taken and given back per call it is mapped afresh
-// around every synchronizing adjoint(): 150x141x133, 16 steps, 7.1 ms a shot
-// against 5.3.
-int ensure_t1_scratch(tti_sim* s)
-{
-    if (s->cfg.scheme != 1 || s->cfg.fused || s->base) return TTI_OK;
-    return s->alloc((void**)&s->base, (size_t)s->nvol() * sizeof(float4));
 }
 
 int adjoint_per_kernel_step(tti_sim* s, cudaStream_t st)
@@ -1016,8 +1011,9 @@ int tti::sim_create_in_pool(const tti_sim_config* cfg, cudaMemPool_t pool, tti_s
         for (float** v : {&s->rhs3, &s->rhs4, &s->snp, &s->snq, &s->d[0], &s->d[1], &s->d[2], &s->d[3], &s->d[4],
                           &s->d[5]})
             if (!rc) rc = s->alloc((void**)v, vb);
-        if (!rc) rc = s->alloc((void**)&s->base, (size_t)s->nvol() * sizeof(float4));
     }
+    if (!rc && (pl.need_aux || pl.t1_scratch))
+        rc = s->alloc((void**)&s->base, (size_t)s->nvol() * sizeof(float4));
     if (!rc) rc = s->alloc((void**)&s->err, sizeof(int));
     if (!rc) rc = sim_zero(s, s->err, sizeof(int));
     if (!rc) rc = s->alloc((void**)&s->grad_vp, s->ninterior * sizeof(float));
@@ -1303,8 +1299,7 @@ static int sim_adjoint(tti_sim* s, const float* residual, int residual_on_device
     cudaStream_t st0 = s->stream;
     s->launches = 0;
     s->st_mode = 0;
-    int rc = ensure_t1_scratch(s);
-    if (!rc) rc = zero_state(s, s->w);
+    int rc = zero_state(s, s->w);
     if (!rc) rc = sim_zero(s, s->grad_vp, s->ninterior * sizeof(float));
     if (!rc) rc = sim_zero(s, s->grad_rho, s->ninterior * sizeof(float));
     if (rc) return rc;
@@ -1426,8 +1421,7 @@ int tti_sim_adjoint_begin(tti_sim* s, const float* residual, int residual_on_dev
     const tti_sim_config& c = s->cfg;
     s->launches = 0;
     s->st_mode = 0;
-    int rc = ensure_t1_scratch(s);
-    if (!rc) rc = zero_state(s, s->w);
+    int rc = zero_state(s, s->w);
     if (!rc) rc = sim_zero(s, s->grad_vp, s->ninterior * sizeof(float));
     if (!rc) rc = sim_zero(s, s->grad_rho, s->ninterior * sizeof(float));
     if (!rc && s->nrec) {

@@ -127,6 +127,14 @@ def test_scheme_is_validated_and_type1_needs_no_derivative_volumes():
     assert P.Config(**base, scheme=1).footprint_bytes() == fused - 8 * vol
 
 
+def test_footprint_holds_the_centred_launchers_adjoint_scratch():
+    """Four volumes beside the fused path's plan, where there is an adjoint
+    pass (it needs snapshots)."""
+    cfg = dict(nx=64, ny=64, nz=64, nt=40, xcorr_step=4, scheme=1)
+    vol = 96 * 72 * 72 * 4
+    assert P.Config(**cfg, fused=False).footprint_bytes() - P.Config(**cfg).footprint_bytes() == 4 * vol
+
+
 def test_type1_snapshot_slots_hold_two_fields():
     n = 64 * 64 * 64
     cfg = dict(nx=64, ny=64, nz=64, nt=400, xcorr_step=4, scheme=1)

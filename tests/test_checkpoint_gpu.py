@@ -72,3 +72,27 @@ def test_footprint_matches_device_allocation():
     sim.close()
     used = free0 - free1
     assert want <= used <= want + 64 * 2**20
+
+
+@pytest.mark.gpu
+def test_footprint_covers_a_whole_shot_of_the_centred_launchers():
+    """What the simulator holds after forward() and adjoint() is what its plan
+    says: nothing is taken on the way."""
+    import torch
+    nt = 4
+    nx, ny, nz = 256, 224, 224
+    cfg = P.Config(nx=nx, ny=ny, nz=nz, nt=nt, scheme=1, fused=False, dt=1e-3)
+    want = cfg.footprint_bytes()
+    torch.cuda.synchronize()
+    free0, _ = torch.cuda.mem_get_info()
+    sim = P.Simulator(cfg)
+    sim.set_model(vp=np.full((nz, ny, nx), 2000.0, np.float32))
+    sim.set_source(nx // 2, ny // 2, 5, np.ones(nt, np.float32))
+    sim.forward()
+    sim.adjoint(np.zeros((nt, 0), np.float32))
+    torch.cuda.synchronize()
+    free1, _ = torch.cuda.mem_get_info()
+    sim.close()
+    # the scratch alone is 248 MB; the allocator maps in steps of 32 MiB and
+    # may keep what the model upload (one parameter, 51 MB) gave back
+    assert want <= free0 - free1 <= want + 128 * 2**20
