@@ -2225,15 +2225,6 @@ bool layout_supported(const Layout& L)
            L.ldimz == L.izend + 1 + kRadius;
 }
 
-int device_sms()
-{
-    int sms = 148;
-    int dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaGetLastError();
-    return sms;
-}
-
 long long work_planes(const Layout& L)
 {
     return (long long)((L.nx() + TX - 1) / TX) * ((L.ny() + TY - 1) / TY) * L.nz();
@@ -2281,8 +2272,8 @@ std::vector<int> plane_candidates(const Layout& L)
 // of the type1 forward kernel's 256-thread CTAs, one of the others.
 int kind_ctas_per_sm(int kind) { return kind == KIND_T1F ? 2 : 1; }
 
-// Modelled time of a step, in plane-iterations of the slowest CTA: per_sm
-// resident CTAs per SM, each segment pays the 2*lag-plane pipeline fill
+// Modelled time of a step, in plane-iterations of the slowest CTA: slots
+// resident CTAs, each segment pays the 2*lag-plane pipeline fill
 // (weighed, see fill_weight), a range of bz planes covers at most
 // ceil((bz-1)/nz)+1 columns (one when whole columns divide evenly).
 //
@@ -2295,11 +2286,10 @@ int kind_ctas_per_sm(int kind) { return kind == KIND_T1F ? 2 : 1; }
 // (forward 13/14: 62 us against 73 us with 11/22).
 double fill_weight(int kind) { return kind == KIND_FWD ? 0.3 : 0.55; }
 
-double plane_cost(const Layout& L, int bz, double lag, int per_sm)
+double plane_cost(const Layout& L, int bz, double lag, long long slots)
 {
     const int nz = L.nz();
     const long long ctas = cta_count(L, Split{bz, 0});
-    const long long slots = (long long)device_sms() * per_sm;
     const double waves = (double)((ctas + slots - 1) / slots);
     int segs;
     if (bz <= nz && nz % bz == 0)
@@ -2327,11 +2317,10 @@ bool column_aligned(const Layout& L, int bz) { return bz <= L.nz() && L.nz() % b
 // Modelled cost of a top/bottom split in one wave: the tops (one segment
 // each) against the bottom CTAs, whose bz planes cross at most
 // ceil((bz-1)/span)+1 column bottoms.
-double split_cost(const Layout& L, Split sp, double lag, int per_sm)
+double split_cost(const Layout& L, Split sp, double lag, long long slots)
 {
     const int span = L.nz() - sp.ztop;
     const int segs = (sp.bz - 1) / span + 2;
-    const long long slots = (long long)device_sms() * per_sm;
     const double waves = (double)((cta_count(L, sp) + slots - 1) / slots);
     return waves * std::max(sp.ztop + 2.0 * lag, sp.bz + 2.0 * lag * segs);
 }
@@ -2373,18 +2362,18 @@ Split pick_split(const Layout& L, int kind)
     double best_cost = 1e300;
     const bool any_split = kind == KIND_FWD || kind == KIND_T1F;  // few staged arrays
     const double lag = fill_weight(kind) * kind_lag(kind);
-    const int per_sm = kind_ctas_per_sm(kind);
+    const long long slots = (long long)device_sms() * kind_ctas_per_sm(kind);
     for (int bz : plane_candidates(L)) {
         const bool aligned = column_aligned(L, bz);
         if (!any_split && !aligned) continue;
-        const double cost = plane_cost(L, bz, lag, per_sm) * (aligned ? 1.0 : 1.2);
+        const double cost = plane_cost(L, bz, lag, slots) * (aligned ? 1.0 : 1.2);
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = Split{bz, 0};
         }
     }
     for (const Split& sp : topbottom_candidates(L, kind)) {
-        const double cost = split_cost(L, sp, lag, per_sm);
+        const double cost = split_cost(L, sp, lag, slots);
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = sp;
@@ -2394,6 +2383,24 @@ Split pick_split(const Layout& L, int kind)
 }
 
 } // namespace
+
+int device_sms()
+{
+    static std::atomic<int> count[kMaxDevices];  // 0: not asked yet
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
+        cudaGetLastError();
+        return 148;
+    }
+    sms = count[dev].load(std::memory_order_relaxed);
+    if (sms > 0) return sms;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+        cudaGetLastError();
+        return 148;
+    }
+    count[dev].store(sms, std::memory_order_relaxed);
+    return sms;
+}
 
 inline float2 pair(float c) { return make_float2(c, c); }
 

@@ -174,6 +174,10 @@ struct ImageArgs {
 bool fused_image_supported(const Layout& L);
 int launch_fused_image(const Layout& L, const ImageArgs& a, cudaStream_t st);
 
+// SMs of the current device (148 where there is none), asked for once per
+// device: the untuned launches choose their split, and so come here, each time.
+int device_sms();
+
 // Status of the bounded waits inside the fused kernels since the last call
 // (TTI_ETIMEOUT if any gave up, TTI_ERANGE if a reduced-precision snapshot
 // saturated); synchronizes the stream and clears the word.  word = nullptr
@@ -200,9 +204,9 @@ Split choose_split(const Layout& L, int kind);
 void record_tuned_split(const Layout& L, int kind, Split s);  // bz = 0 clears
 Split tuned_split(const Layout& L, int kind);                 // bz = 0 if none recorded
 Split model_split(const Layout& L, int kind);
-// Candidates the tuner tries: whole-column chunks ceil(nz/n), equal shares
-// of the work for 1..8 CTAs per SM (each at least 8 planes), and top/bottom
-// splits around the balance point of the kind's pipeline fill.
+// Candidates the tuner tries: whole-column chunks ceil(nz/n) of at least 2
+// planes, equal shares of the work for 1..8 CTAs per SM (each at least 8
+// planes), and top/bottom splits around the balance point of the kind's pipeline fill.
 std::vector<Split> split_candidates(const Layout& L, int kind);
 
 // Type1 scheme (constant density, centred second derivatives): fused forward
