@@ -321,8 +321,8 @@ int tti_selfcheck_bounded_wait(double seconds, tti_stream_t stream);
  * or more column segments, each paying a pipeline fill of 14 planes), so bz
  * sets how many CTAs a step launches against the fill overhead.
  * tti_sim_autotune times every candidate split (whole-column chunks
- * ceil(nz/n), equal shares for 1..8 CTAs per SM of at least 8 planes, and,
- * on grids with fewer tile columns than SMs, top/bottom splits as for
+ * ceil(nz/n) of at least 8 planes (2 on grids whose 8-plane chunks leave SMs
+ * idle), equal shares for 1..8 CTAs per SM of at least 8 planes, and, on grids with fewer tile columns than SMs, top/bottom splits as for
  * tti_tune_set_split around the balance point of the tops) of the fused
  * forward, adjoint and (with a snapshot store) imaging kernels on this
  * simulator's volumes, reps launches each, times the three fastest (and the

@@ -2240,25 +2240,32 @@ unsigned cta_count(const Layout& L, Split sp)
     return (unsigned)(T + (T * (L.nz() - sp.ztop) + sp.bz - 1) / sp.bz);
 }
 
-// Planes per CTA worth trying: whole-column chunks ceil(nz/n) of at least 2
-// planes, and shares of at least 8 that give every SM one, two, ... equal
-// parts of the work.  A 2-plane chunk computes 2 planes out of 16, yet on a
-// grid of few columns the SMs would otherwise idle: 48x40x40 (6 columns), 2
-// planes against 8: forward 21 against 38 us, adjoint 41 against 59 us,
-// imaging 47 against 64 us; a chunk of 1 plane (two waves) is slower again
-// (74 us adjoint).
-std::vector<int> plane_candidates(const Layout& L)
+// CTAs of a kind resident per SM: shared memory (and registers) allow two
+// of the type1 forward kernel's 256-thread CTAs, one of the others.
+int kind_ctas_per_sm(int kind) { return kind == KIND_T1F ? 2 : 1; }
+
+// Planes per CTA worth trying: whole-column chunks ceil(nz/n), and shares of
+// at least 8 that give every SM one, two, ... equal parts of the work.
+// Chunks are of at least 8 planes, too, except on grids whose 8-plane chunks
+// leave SMs idle.  There a 2-plane chunk computes 2 planes out of 16, yet
+// fills the SMs: 48x40x40 (6 columns), 2 planes against 8: forward 25 against
+// 40 us, adjoint 27 against 43 us, imaging 25 against 39 us; a chunk of 1
+// plane (two waves) is slower again (74 us adjoint).  Elsewhere shorter chunks
+// only add waves that each pay their fill, and the tuner would time them all
+// (256^3: the first pass over the chunks 1.6 times as long).
+std::vector<int> plane_candidates(const Layout& L, int kind)
 {
     std::vector<int> c;
-    const int nz = L.nz();
+    const int nz = L.nz(), sms = device_sms();
+    const bool idle = tile_count(L) * ((nz + 7) / 8) < (long long)sms * kind_ctas_per_sm(kind);
+    const int least = idle ? 2 : 8;
     for (int nch = 1; nch <= nz; ++nch) {
         const int bz = (nz + nch - 1) / nch;
-        if (bz < 2 && nch > 1) break;
+        if (bz < least && nch > 1) break;
         c.push_back(bz);
         if (nz % nch == 0) c.push_back(nz / nch);
     }
     const long long W = work_planes(L);
-    const int sms = device_sms();
     for (int k = 1; k <= 8; ++k) {
         const long long b = (W + (long long)sms * k - 1) / ((long long)sms * k);
         if (b >= 8 && b <= (1LL << 30)) c.push_back((int)b);
@@ -2267,10 +2274,6 @@ std::vector<int> plane_candidates(const Layout& L)
     c.erase(std::unique(c.begin(), c.end()), c.end());
     return c;
 }
-
-// CTAs of a kind resident per SM: shared memory (and registers) allow two
-// of the type1 forward kernel's 256-thread CTAs, one of the others.
-int kind_ctas_per_sm(int kind) { return kind == KIND_T1F ? 2 : 1; }
 
 // Modelled time of a step, in plane-iterations of the slowest CTA: slots
 // resident CTAs, each segment pays the 2*lag-plane pipeline fill
@@ -2363,7 +2366,7 @@ Split pick_split(const Layout& L, int kind)
     const bool any_split = kind == KIND_FWD || kind == KIND_T1F;  // few staged arrays
     const double lag = fill_weight(kind) * kind_lag(kind);
     const long long slots = (long long)device_sms() * kind_ctas_per_sm(kind);
-    for (int bz : plane_candidates(L)) {
+    for (int bz : plane_candidates(L, kind)) {
         const bool aligned = column_aligned(L, bz);
         if (!any_split && !aligned) continue;
         const double cost = plane_cost(L, bz, lag, slots) * (aligned ? 1.0 : 1.2);
@@ -2855,7 +2858,7 @@ Split choose_split(const Layout& L, int kind)
 std::vector<Split> split_candidates(const Layout& L, int kind)
 {
     std::vector<Split> c;
-    for (int bz : plane_candidates(L)) c.push_back(Split{bz, 0});
+    for (int bz : plane_candidates(L, kind)) c.push_back(Split{bz, 0});
     for (const Split& sp : topbottom_candidates(L, kind)) c.push_back(sp);
     return c;
 }

@@ -204,9 +204,9 @@ Split choose_split(const Layout& L, int kind);
 void record_tuned_split(const Layout& L, int kind, Split s);  // bz = 0 clears
 Split tuned_split(const Layout& L, int kind);                 // bz = 0 if none recorded
 Split model_split(const Layout& L, int kind);
-// Candidates the tuner tries: whole-column chunks ceil(nz/n) of at least 2
-// planes, equal shares of the work for 1..8 CTAs per SM (each at least 8
-// planes), and top/bottom splits around the balance point of the kind's pipeline fill.
+// Candidates the tuner tries: whole-column chunks ceil(nz/n), equal shares
+// of the work for 1..8 CTAs per SM (each at least 8 planes; chunks down to 2
+// where 8-plane chunks leave SMs idle), and top/bottom splits around the balance point of the kind's pipeline fill.
 std::vector<Split> split_candidates(const Layout& L, int kind);
 
 // Type1 scheme (constant density, centred second derivatives): fused forward

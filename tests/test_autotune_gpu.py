@@ -65,3 +65,25 @@ def test_chunk_length_does_not_change_results_and_tuner_records_a_choice():
     finally:
         for k in P.TUNE_KINDS:
             P.tune_set(NX, NY, NZ, k, 0)
+
+
+@pytest.mark.gpu
+def test_tuner_leaves_out_short_chunks_where_longer_ones_fill_the_gpu():
+    """640x240x32 has 300 tile columns, more than two for each SM: the tuner
+    tries the whole-column chunks of 8 planes and more and the equal shares,
+    and no top/bottom split."""
+    import torch
+
+    nx, ny, nz = 640, 240, 32
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    tiles = -(-nx // 32) * -(-ny // 16)
+    assert tiles > 2 * sms
+    want = {-(-nz // n) for n in range(1, nz // 8 + 1)}
+    want |= {b for b in (-(-tiles * nz // (sms * k)) for k in range(1, 9)) if b >= 8}
+    try:
+        with P.Simulator(P.Config(nx=nx, ny=ny, nz=nz, nt=4, dt=1e-3, save_snapshots=False)) as sim:
+            sim.set_model(vp=np.full((nz, ny, nx), 2000.0, np.float32))
+            assert sim.autotune(reps=1)["candidates"] == len(want)
+    finally:
+        for k in P.TUNE_KINDS:
+            P.tune_set(nx, ny, nz, k, 0)
