@@ -2280,14 +2280,29 @@ std::vector<int> plane_candidates(const Layout& L, int kind)
 // (weighed, see fill_weight), a range of bz planes covers at most
 // ceil((bz-1)/nz)+1 columns (one when whole columns divide evenly).
 //
-// A fill plane counts fill_weight of an output's plane: it has no output
-// stage, in the forward kernel (which does its in-plane work there) hardly more
-// than the mixed terms, and the imaging and short-chunk adjoint kernels skip
-// most of it.  With these weights the model chooses what the autotuner does at
-// 256^3 (adjoint and imaging 148/233, forward 199/225; a weight of 1 gave
-// 96/241, 2 % slower), 224x224x160 (forward 104/107, 2 %) and 101x93x77
-// (forward 13/14: 62 us against 73 us with 11/22).
-double fill_weight(int kind) { return kind == KIND_FWD ? 0.3 : 0.55; }
+// A fill plane counts fill_weight of an output's plane.  The forward kernel
+// does its in-plane work with the output, the imaging and short-chunk adjoint
+// kernels skip most of it on fill planes; the type1 forward has next to nothing
+// to do on one, while the type1 adjoint forms and scatters it in full.  Slopes
+// measured at 48x40x40 (time against chunk length): forward 0.38 (VTI) to
+// 0.47, adjoint 0.49 to 0.59, imaging 0.51, type1 forward 0.36, type1 adjoint
+// 1.1.  The weights are those that chose best over 40 grids of 32 to 512 cells
+// per side (a little below the slopes, because the bottoms' segments are counted
+// at their most), checked on 46 others.  Time of the choice over the fastest
+// candidate timed, geometric mean of the 86 (and worst): forward 1.006 (1.18),
+// adjoint 1.002 (1.07), imaging 1.001 (1.04), type1 forward 1.004 (1.12), type1
+// adjoint 1.000 (1.01).  A weight of 1 throughout, on chunks of 8 planes and
+// more, gave 1.16, 1.10, 1.10, 1.19, 1.04.
+double fill_weight(int kind)
+{
+    switch (kind) {
+    case KIND_FWD: return 0.3;
+    case KIND_ADJ: return 0.4;
+    case KIND_IMG: return 0.35;
+    case KIND_T1F: return 0.2;
+    default: return 0.8;
+    }
+}
 
 double plane_cost(const Layout& L, int bz, double lag, long long slots)
 {
@@ -2310,11 +2325,13 @@ double plane_cost(const Layout& L, int bz, double lag, long long slots)
 // them.  Unaligned shares balance the SMs better but spread the CTAs over
 // all of z; a kernel that stages many halo'd arrays then re-reads its halos
 // from HBM (the adjoint stages nine, the imaging kernel eleven).  The forward
-// kernels stage three and two: an unaligned share counts 1.2 times its
+// kernels stage three and two: an unaligned share counts 1.1 times its
 // modelled cost for them.  512x512x400: 2.47 ms in aligned shares of 200
 // planes, 2.96 ms in unaligned ones of 1384, which the model alone puts 3 %
-// below; 256^3: 611 us top/bottom (199/225), 607 us in unaligned shares of
-// 222 planes with twice the DRAM bytes.
+// below; 256^3: 643 us top/bottom (199/225), 646 us in unaligned shares of
+// 222 planes with twice the DRAM bytes (VTI 442, 526).  More would refuse good
+// ones: 296x300x40, 188 us in shares of 52 planes (VTI 133), 209 in aligned
+// ones of 20 (140), which a handicap of 1.2 takes.
 bool column_aligned(const Layout& L, int bz) { return bz <= L.nz() && L.nz() % bz == 0; }
 
 // Modelled cost of a top/bottom split in one wave: the tops (one segment
@@ -2369,7 +2386,7 @@ Split pick_split(const Layout& L, int kind)
     for (int bz : plane_candidates(L, kind)) {
         const bool aligned = column_aligned(L, bz);
         if (!any_split && !aligned) continue;
-        const double cost = plane_cost(L, bz, lag, slots) * (aligned ? 1.0 : 1.2);
+        const double cost = plane_cost(L, bz, lag, slots) * (aligned ? 1.0 : 1.1);
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = Split{bz, 0};

@@ -163,6 +163,22 @@ def test_work_split_table_round_trip():
             P.tune_set(64, 48, 40, k, 0)
 
 
+@pytest.mark.parametrize("grid,kind,split", [
+    ((296, 300, 40), "forward", (52, 0)),        # 188 us; aligned 20-plane shares 209
+    ((400, 300, 60), "forward", (101, 0)),       # 322 us; (60, 0) 358
+    ((512, 512, 400), "forward", (200, 0)),      # unaligned shares cost DRAM bytes here
+    ((264, 46, 42), "adjoint", (8, 10)),         # 50 us; (14, 0) 60
+    ((264, 46, 42), "imaging", (8, 10)),         # 43 us; (14, 0) 54
+    ((280, 292, 32), "type1_forward", (19, 0)),  # 88 us; (13, 23) 97
+    ((120, 46, 106), "type1_forward", (5, 0)),   # 30 us; (4, 12) 38
+    ((96, 33, 76), "type1_adjoint", (5, 13)),    # 47 us; (4, 0) 51
+    ((264, 46, 42), "type1_adjoint", (14, 0)),   # 49 us; (8, 9) 51
+    ((48, 40, 40), "adjoint", (2, 0)),           # 27 us; 8-plane chunks 43
+])
+def test_modelled_split_is_the_one_that_measured_faster(grid, kind, split):
+    assert P.tune_get_split(*grid, kind) == split
+
+
 def test_wave_precision_is_validated_and_costs_only_its_scales():
     base = dict(nx=64, ny=64, nz=64, nt=40, xcorr_step=4, save_snapshots=False)
     with pytest.raises(P.TTIError) as e:
