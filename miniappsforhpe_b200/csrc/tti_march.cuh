@@ -7,6 +7,7 @@
 #pragma once
 
 #include "tti_common.cuh"
+#include "tti_internal.cuh"
 
 namespace tti {
 
@@ -105,19 +106,27 @@ inline dim3 march_grid(const MarchArgs& a)
     return dim3((a.ixend - a.ixbeg + MX) / MX, (a.iyend - a.iybeg + MY) / MY, (a.izend - a.izbeg + a.bz) / a.bz);
 }
 
-// Output planes per block: the cut of the columns into n chunks (of at least 8
-// planes) with the least work on the last SM, one block resident on each of
-// the 148 and each chunk paying the planes around it, which form and scatter
-// about half of what an output's plane does.
+// Output planes per block: the cut of the columns into n chunks with the least
+// work on the last SM, one block resident on each and each chunk paying the
+// planes around it, which form and scatter about half of what an output's plane
+// does.  Chunks of less than 8 planes only while all blocks fit at once: on
+// small grids the SMs are idle otherwise, and a march is as long as its chunk.
+// Calls with their temporaries' kernel, 8 planes at least -> as here (a thread
+// per cell): 48x40x40 adjoint derivatives 27.7 -> 16.6 us (19.2), density
+// gradient 23.0 -> 11.7 (10.1), type1 adjoint 28.4 -> 15.6 (13.5); 64^3 28.7 ->
+// 21.3 (37.8), 24.0 -> 16.4 (23.1), 29.5 -> 20.9 (27.8); 20^3, nine planes for
+// one of output, 29.2 -> 13.7 (11.5), 26.3 -> 9.3 (9.8), 30.1 -> 12.4 (11.1).
+// From 80^3 on the cut is as before.
 inline int march_bz(int nx, int ny, int nz)
 {
-    const int64_t tiles = (int64_t)((nx + MX - 1) / MX) * ((ny + MY - 1) / MY);
+    const int64_t tiles = (int64_t)((nx + MX - 1) / MX) * ((ny + MY - 1) / MY), sms = device_sms();
     int best = nz;
     double least = 1e300;
-    for (int n = 1; n == 1 || n <= nz / 8; ++n) {
+    for (int n = 1; n <= nz; ++n) {
         const int bz = (nz + n - 1) / n;
         const int64_t blocks = tiles * ((nz + bz - 1) / bz);
-        const double cost = (double)((blocks + 147) / 148) * (bz + 0.5 * 2 * kRadius);
+        if (n > 1 && n > nz / 8 && blocks > sms) break;
+        const double cost = (double)((blocks + sms - 1) / sms) * (bz + 0.5 * 2 * kRadius);
         if (cost < least - 1e-9) {
             least = cost;
             best = bz;

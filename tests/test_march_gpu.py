@@ -1,7 +1,7 @@
 """The marching launchers (adjoint derivatives, density gradient, type1 adjoint)
-at the edges of their tiles and chunks: extents around 32 columns, 16 rows and
-the 8-plane chunk limit, single cells, and ranges inside a larger allocation,
-against the oracle.  Tolerance: FP32 rounding of one kernel's sums, the same
+at the edges of their tiles and chunks: extents around 32 columns and 16 rows,
+chunks of 1 to 3 planes (small grids) and of 13 with a remainder (91 tiles x 37
+planes), single cells, and ranges inside a larger allocation, against the oracle.  Tolerance: FP32 rounding of one kernel's sums, the same
 2e-6 relative L2 as the other launcher tests."""
 import numpy as np
 import pytest
@@ -12,7 +12,8 @@ from tests.helpers import random_field, random_model, rel_l2, sponge_ab
 
 H, DT, TOL = (10.0, 12.5, 8.0), 1e-3, 2e-6
 DK = ("d1x", "d1y", "d1z", "d2x", "d2y", "d2z")
-DIMS = ((1, 1, 1), (31, 15, 7), (32, 16, 8), (33, 17, 9), (65, 3, 130), (5, 50, 16), (40, 33, 17))
+DIMS = ((1, 1, 1), (31, 15, 7), (32, 16, 8), (33, 17, 9), (65, 3, 130), (5, 50, 16), (40, 33, 17),
+        (48, 40, 41), (200, 200, 37))
 
 
 def dev(a):
