@@ -213,6 +213,7 @@ constexpr int E3PY = 2 * E3Y;
 struct E3Pre {
     const float* in[6];
     float *xz[6], *yz[6];
+    int b0;  // first z block of this launch
 };
 
 template <int XS, int YS, int ZS, int V>
@@ -282,7 +283,7 @@ template <int V>
 __global__ void __launch_bounds__(E3X* E3Y) k_e3_precompute(E3Pre a, E3Grid g)
 {
     __shared__ __align__(16) float t[3][E3PY + 8][E3X + 8];
-    const int v = blockIdx.z % 6, b = blockIdx.z / 6;
+    const int v = blockIdx.z % 6, b = a.b0 + blockIdx.z / 6;
     if (v < 3)
         e3_precompute<1, 1, 1, V>(t, a.in[v], a.xz[v], a.yz[v], g, b);
     else if (v == 3)
@@ -601,14 +602,19 @@ int tti_e3_launch_splain(float* f4, float* f5, float* f6, float* f7, float* f8, 
     const E3Grid g{nx, ny, nz, ldimx, ldimy};
     cudaStream_t st = S(stream);
     // the six z-mixed precomputes of sPlainLoop (simulator3SetUp.cu:1177-1186)
-    const dim3 pb((nx + E3X - 1) / E3X, (ny + E3PY - 1) / E3PY, 6 * ((nz - 1) / 64 + 1)), t(E3X, E3Y);
+    const dim3 t(E3X, E3Y);
     float* const* p = f10_21;
-    const E3Pre pre{{f1_1, f2_2, f3_3, f1_2, f1_3, f2_3}, {p[0], p[6], p[10], p[2], p[4], p[8]},
-                    {p[1], p[7], p[11], p[3], p[5], p[9]}};
-    if (vec4_ok(ldimx, {f1_1, f2_2, f3_3, f1_2, f1_3, f2_3}))
-        k_e3_precompute<4><<<pb, t, 0, st>>>(pre, g);
-    else
-        k_e3_precompute<1><<<pb, t, 0, st>>>(pre, g);
+    E3Pre pre{{f1_1, f2_2, f3_3, f1_2, f1_3, f2_3}, {p[0], p[6], p[10], p[2], p[4], p[8]},
+              {p[1], p[7], p[11], p[3], p[5], p[9]}, 0};
+    const bool pre4 = vec4_ok(ldimx, {f1_1, f2_2, f3_3, f1_2, f1_3, f2_3});
+    constexpr int most = 65535 / 6;  // z blocks of the six volumes in one launch
+    for (const int nb = (nz - 1) / 64 + 1; pre.b0 < nb; pre.b0 += most) {
+        const dim3 pb((nx + E3X - 1) / E3X, (ny + E3PY - 1) / E3PY, 6 * (nb - pre.b0 < most ? nb - pre.b0 : most));
+        if (pre4)
+            k_e3_precompute<4><<<pb, t, 0, st>>>(pre, g);
+        else
+            k_e3_precompute<1><<<pb, t, 0, st>>>(pre, g);
+    }
     E3Stress a{};
     float* out[6] = {f4, f5, f6, f7, f8, f9};
     a.f4 = out[0];

@@ -208,3 +208,24 @@ def test_stress_update_on_rows_of_odd_length():
         assert maxerr(a[I], b[I]) < 1e-5
     for a, b in zip(host(gs), s_o):
         assert maxerr(a, b) < 1e-5
+
+
+def test_stress_update_of_more_z_blocks_than_one_launch_of_the_precomputes_holds():
+    """10924 blocks of 64 planes, six volumes each, pass the 65535 of a
+    launch's z extent; the last three blocks (the last with 28 planes), where
+    the second launch begins, are those of the same planes alone."""
+    from miniappsforhpe_b200 import elastic as E
+
+    nz, first = 10923 * 64 + 28, 10921 * 64
+    gen = torch.Generator(device="cuda").manual_seed(16)
+    new = lambda: torch.randn((nz + 8, 9, 9), generator=gen, device="cuda")
+    M, d, s = [new()] * 21, [new(), new()] * 3, [new() for _ in range(6)]
+    pre = [torch.zeros_like(s[0]) for _ in range(12)]
+    tail = lambda fs: [f[first:].clone() for f in fs]
+    s_t, pre_t = tail(s), tail(pre)
+    E.launch_splain(*s_t, tail(M[:1]) * 21, *tail(d), pre_t, 1, 1, nz - first, 9, 9)
+    E.launch_splain(*s, M, *d, pre, 1, 1, nz, 9, 9)
+    torch.cuda.synchronize()
+    for whole, part in zip(s + pre, s_t + pre_t):
+        assert float(part[4:-4, 4, 4].abs().min()) > 0
+        assert torch.equal(whole[first + 4:-4], part[4:-4])
