@@ -229,3 +229,35 @@ def test_stress_update_of_more_z_blocks_than_one_launch_of_the_precomputes_holds
     for whole, part in zip(s + pre, s_t + pre_t):
         assert float(part[4:-4, 4, 4].abs().min()) > 0
         assert torch.equal(whole[first + 4:-4], part[4:-4])
+
+
+# The velocity and strain kernels walk 64 planes per block where that leaves
+# six blocks for each SM, else 32 or 16 (every grid above): tile columns enough
+# for 64 (462) and for 32 (320), nz = 70 leaving a remainder of 6 planes.
+@pytest.mark.parametrize("nx,ny", [(672, 176), (512, 160)], ids=["64", "32"])
+def test_velocity_kernels_in_long_chunks(nx, ny):
+    from miniappsforhpe_b200 import elastic as E
+
+    lay = Layout(nx, ny, 70)
+    rng = np.random.default_rng(17)
+    v, s, (M22,), zp = vols(3, rng, lay), vols(6, rng, lay), vols(1, rng, lay), zprime_of(lay)
+    e = ElasticOracle()
+    d = [lay.zeros() for _ in range(6)]
+    e.vgplain(lay, *v, d, zp)
+    v_o = [x.copy() for x in v]
+    e.vplain(lay, v_o, s, M22, zp)
+
+    def run(nx, ny):
+        gv, gd, gz = dev(v), dev([lay.zeros() for _ in range(6)]), torch.from_numpy(zp).cuda()
+        E.launch_vgplain(*gv, *gd, gz, nx, ny, lay.nz, lay.ldimx, lay.ldimy)
+        E.launch_vplain(*gv, *dev(s), torch.from_numpy(M22).cuda(), gz, nx, ny, lay.nz, lay.ldimx, lay.ldimy)
+        torch.cuda.synchronize()
+        return host(gv + gd)
+
+    long = run(nx, ny)
+    for a, b in zip(long, v_o + d):
+        assert maxerr(a, b) < 1e-5
+    # the first columns again, few enough for 16-plane chunks: the same bits
+    inside = (slice(4, 4 + lay.nz), slice(4, 4 + 24), slice(4, 4 + 64))
+    for a, b in zip(long, run(64, 24)):
+        np.testing.assert_array_equal(a[inside], b[inside])
