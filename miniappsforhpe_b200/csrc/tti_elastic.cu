@@ -24,6 +24,7 @@
 #include <cuda_pipeline.h>
 
 #include "tti_common.cuh"
+#include "tti_internal.cuh"
 
 namespace tti {
 namespace {
@@ -49,14 +50,14 @@ struct E3Grid {
 };
 
 // Planes per block of the z-windowed kernels: the most that leaves six blocks
-// for each of the 148 SMs, 16 at least (a chunk starts with eight planes of
+// for each SM, 16 at least (a chunk starts with eight planes of
 // window loads).  211x187x150 (504 blocks of 64 planes): velocity update 135 -> 107 us,
 // strains 97 -> 79 us.
 int e3_zchunk(const E3Grid& g)
 {
     const int64_t columns = (int64_t)((g.nx + E3X - 1) / E3X) * ((g.ny + E3Y - 1) / E3Y);
     int zper = E3ZC;
-    while (zper > 16 && columns * ((g.nz + zper - 1) / zper) < 6 * 148) zper /= 2;
+    while (zper > 16 && columns * ((g.nz + zper - 1) / zper) < 6 * device_sms()) zper /= 2;
     return zper;
 }
 
@@ -118,7 +119,7 @@ __device__ __forceinline__ void stage_tile_async(float (&t)[R][C], const float* 
 }
 
 // vgPlainKernel (simulator3SetUp.cu:1218-1362): the six strain volumes.  A
-// block walks E3ZC planes of a 32x8 column tile: the x/y taps of each plane
+// block walks zper planes of a 32x8 column tile: the x/y taps of each plane
 // come from shared-memory tiles of f1, f2, f3 with a halo of 4, the z taps
 // from per-thread register windows (one load per plane and field), as the
 // reference's shared planes and queues do.
@@ -395,8 +396,10 @@ __global__ void __launch_bounds__(E3X* E3Y, 2) k_e3_splain(E3Stress a, E3Grid g)
 // each plane, z taps of f6, f8, f9 from register windows, and M22 of the
 // plane below kept from the previous plane; M22 (with the row above and
 // the columns left of the tile) and the three velocities it updates come
-// through shared tiles of the plane too.
-template <int V>
+// through shared tiles of the plane too.  ZPER: the chunk length when it is the
+// longest (0: zper): as a constant there it schedules better (256^3 260 -> 257
+// us; the strains gain nothing, and shorter chunks lose).
+template <int V, int ZPER>
 __global__ void __launch_bounds__(E3X* E3Y) k_e3_vplain(float* __restrict__ f1, float* __restrict__ f2,
                                                        float* __restrict__ f3, const float* __restrict__ f4,
                                                        const float* __restrict__ f5, const float* __restrict__ f6,
@@ -416,7 +419,8 @@ __global__ void __launch_bounds__(E3X* E3Y) k_e3_vplain(float* __restrict__ f1, 
     const bool act = ix < 4 + g.nx && iy < 4 + g.ny;
     const float invd1 = 1.01f, invd2 = 2.01f;
     const int64_t sz = (int64_t)g.ldimx * g.ldimy;
-    const int z0 = 4 + blockIdx.z * zper, z1 = min(z0 + zper, 4 + g.nz);
+    const int zc = ZPER ? ZPER : zper;
+    const int z0 = 4 + blockIdx.z * zc, z1 = min(z0 + zc, 4 + g.nz);
     float w6[9] = {}, w8[9] = {}, w9[9] = {};  // planes iz-4 .. iz+4
     float m22z = 0.0f;
     if (act) {
@@ -656,12 +660,10 @@ int tti_e3_launch_vplain(float* f1, float* f2, float* f3, const float* f4, const
         return TTI_EINVAL;
     const E3Grid g{nx, ny, nz, ldimx, ldimy};
     const int zper = e3_zchunk(g);
-    if (vec4_ok(ldimx, {f1, f2, f3, f4, f5, f6, f7, f8, f9, M22}))
-        k_e3_vplain<4><<<e3_blocks(g, zper), dim3(E3X, E3Y), 0, S(stream)>>>(f1, f2, f3, f4, f5, f6, f7, f8, f9, M22,
-                                                                             zprime, g, zper);
-    else
-        k_e3_vplain<1><<<e3_blocks(g, zper), dim3(E3X, E3Y), 0, S(stream)>>>(f1, f2, f3, f4, f5, f6, f7, f8, f9, M22,
-                                                                             zprime, g, zper);
+    const bool v4 = vec4_ok(ldimx, {f1, f2, f3, f4, f5, f6, f7, f8, f9, M22});
+    auto* k = zper == E3ZC ? (v4 ? k_e3_vplain<4, E3ZC> : k_e3_vplain<1, E3ZC>)
+                           : (v4 ? k_e3_vplain<4, 0> : k_e3_vplain<1, 0>);
+    k<<<e3_blocks(g, zper), dim3(E3X, E3Y), 0, S(stream)>>>(f1, f2, f3, f4, f5, f6, f7, f8, f9, M22, zprime, g, zper);
     return launch_status();
 }
 
