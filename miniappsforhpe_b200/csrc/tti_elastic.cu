@@ -205,10 +205,10 @@ __global__ void __launch_bounds__(E3X* E3Y) k_e3_vgplain(const float* __restrict
 // The two pairs of a plane that feed slots i and 7 - i are the same cells.
 //
 // All six precomputes are one launch (blockIdx.z = volume x z block): six
-// launches of 1024 blocks each ended in a nearly empty SM, and each waits for
-// memory more than for bandwidth.  A thread owns two rows (8 apart) of a 32x16
-// tile, whose halo costs 1.9 loads per output instead of 2.5.  256^3: the six
-// 520 -> 468 us (12 B/pt each, 31 us at the copy rate; the waits remain).
+// launches of 1024 blocks each ended in a nearly empty SM.  A thread owns two
+// rows (8 apart) of a 32x16 tile, whose halo costs 1.9 loads per output instead
+// of 2.5.  256^3: the six 520 -> 470 us (12 B/pt each, 184 us in all at the copy
+// rate).  Bound by instruction issue: 0.80 of the issue slots, 0.35 of HBM.
 constexpr int E3PY = 2 * E3Y;
 
 struct E3Pre {

@@ -807,7 +807,11 @@ __global__ void __launch_bounds__(NT, 1) k_fused_adjoint(const __grid_constant__
     for (int j = 0; j < 4; ++j) irq[j] = 0.0f;
 
     for (int t = 0; t < ntot; ++t) {
-        // Stage (t+2)%3 was last read in iteration t-1, before its second barrier.
+        // Stage (t+2)%3 was last read in iteration t-1, before its last
+        // barrier: the second, or, on a skipping plane that has none (neither
+        // in-plane nor mixed), the first.  Such a plane must read its stage
+        // and the tiles before the first barrier only, since the copies below
+        // and the next plane's temporaries follow no other.
         if (tid == 0 && t + ADJ_PF < ntot) {
             fence_proxy_async();
             issue(t + ADJ_PF);

@@ -128,8 +128,10 @@ __global__ void __launch_bounds__(T1X* T1Y)
 
 // The adjoint: marching (tti_march.cuh), the z, yz and zx terms of each plane
 // scattered into a register queue of the outputs L-4 .. L+4, the in-plane terms
-// kept beside it and added last, as the reference does.  Bound by its issue
-// slots; 150x141x133: 233 us with a form of the temporaries per tap, 132 us.
+// kept beside it and added last, as the reference does.  Bound by latency (16
+// warps per SM, issue slots 0.34, waiting on the plane loaded ahead, the shared-
+// memory queue and the barriers; HBM 0.14).  150x141x133: 233 us with a form of
+// the temporaries per tap, 132 us.
 template <bool SPONGE>
 __global__ void __launch_bounds__(MNT, 1)
     k_t1_adj(float* __restrict__ f3, float* __restrict__ f4, MarchArgs a, const float2* __restrict__ abx,
