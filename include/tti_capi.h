@@ -268,7 +268,7 @@ typedef struct {
                              (from the previous step's largest |p|, |q|) and are read back exactly;
                              stencils, pdot/qdot and the time update stay FP32.  The rounded
                              values are held in the FP32 arrays (the stencil kernels are
-                             instruction-bound, not byte-bound), so this is the numerics of
+                             latency-bound, not byte-bound), so this is the numerics of
                              FP16/BF16 wavefield storage without its memory saving. */
 } tti_sim_config;
 

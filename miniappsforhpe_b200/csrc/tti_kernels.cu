@@ -257,9 +257,9 @@ __global__ void __launch_bounds__(BX* BY)
 // shared-memory queue, the plane loaded ahead and the barriers (shared-memory
 // pipe 0.50, HBM 0.24; 72 B/pt would take 45 us at 160^3).  Marching
 // (tti_march.cuh) with one form of the temporaries per plane, the planes' z and
-// yz/zx terms scattered into register queues in the reference's order.  160^3: 514 us with a thread per
-// cell forming them at every tap, 187 us marching with two blocks per SM
-// (64 registers, spills), 152 us with one.
+// yz/zx terms scattered into register queues in the reference's order.  160^3:
+// 514 us with a thread per cell forming them at every tap, 187 us marching with
+// two blocks per SM (64 registers, spills), 152 us with one.
 __global__ void __launch_bounds__(MNT, 1)
     k_adj_drv(float* __restrict__ d1x, float* __restrict__ d2x, float* __restrict__ d1y, float* __restrict__ d2y,
               float* __restrict__ d1z, float* __restrict__ d2z, float* __restrict__ rhs3, float* __restrict__ rhs4,
